@@ -18,25 +18,15 @@
 //   warp 2     S issuer.  S(j) = Q.K(j)^T into one of two score buffers in tensor memory
 //              (tcgen05.mma, both operands in shared memory), one step ahead of the softmax.
 //   warp 3     P.V issuer.  O += P(j).V(j) with P read from its own buffer in tensor memory.
-//   warps 4-11 softmax; a thread owns a query row and one half of the 128 score columns.  Steps that contain a
-//              partial or padding block apply the bit mask; steps of full blocks do no mask work.  P is rounded
-//              to the V dtype (line 61); row sums stay in fp32 (line 57).  Finally O / l is staged in the tile's
-//              Q slot and written with one TMA store per warp; a row with no attended key yields 0 (the
-//              reference yields NaN, line 53).
-//
-// Running maxima.  fp16: scores are exponentiated against the row's running reference max in a single pass (base 2,
-// scale folded as in sparse_attn_kernel.py:152; a row's first scores are tried against 0); the reference moves, and O
-// is rescaled in tensor memory, only when a score exceeds it by more than 2^8 (the pass is then redone from the intact
-// scores).  The two threads of a row exchange their maxima every step.  bf16 has the exponent range of fp32: P = exp2(x)
-// with no reference keeps its precision whatever x is, so a tile runs without maxima, without the exchange and its
-// barrier, and is judged once at its end: every row sum in [2^-48, 2^64] (or 0 with no attended key) and every
-// accumulator finite.  A tile that fails goes back to the scheduling warp, which publishes it again, to be done with
-// maxima; its rows are written a second time behind the first store.  The choice depends on the tile's data alone, so a
-// result does not depend on how tiles meet CTAs.
-// Measured on one B200, a call before and after (both stages): B=2 H=32 S=16384 prefix + window + dropout 1326 -> 1256 us,
-// B=2 S=32768 documents 4115 -> 3898 us, the headline shape at p = 0.5 2191 -> 2152 us, at p = 0.9 (lists only) 924 -> 919
-// us, B=4 S=8192 documents 683 -> 670 us: the more steps a tile has, and the fewer of them are masked, the more it gives.
-// What is left there is shared memory: products and loads without any softmax arithmetic take 91 % of a dense launch.
+//   warps 4-11 softmax; a thread owns a query row and one half of the 128 score columns.  Scores
+//              are exponentiated against the row's running reference max in a single pass (base 2,
+//              scale folded as in sparse_attn_kernel.py:152; a row's first scores are tried against
+//              0); the reference moves, and O is rescaled in tensor memory, only when a score
+//              exceeds it by more than 2^8 (the pass is then redone from the intact scores).  Steps that contain a partial or padding block apply
+//              the bit mask; steps of full blocks do no mask work.  P is rounded to the V dtype
+//              (line 61); row sums stay in fp32 (line 57).  Finally O / l is staged in the tile's Q
+//              slot and written with one TMA store per warp; a row with no attended key yields 0
+//              (the reference yields NaN, line 53).
 //
 // Tensor memory (512 columns): score buffers at 0 and 128, O at 256, P buffers at 384 and 448.
 //
@@ -71,10 +61,8 @@ constexpr int kStagesK = 2;          // K tiles in flight in shared memory
 constexpr int kStagesV = 2;          // V tiles in flight in shared memory
 constexpr int kBitStages = 4;        // steps of bit-mask tiles in flight
 constexpr int kTileRing = 4;         // tile indices the scheduling warp may be ahead of the slowest role
-constexpr int kDoneRing = 8;         // tiles whose outcome the scheduling warp may not have looked at yet (at most 6)
 constexpr uint32_t kPanelBytes = 128u * 128u;   // 128 rows x 64 elements x 2 B
 constexpr float kRescaleThreshold = 8.0f;       // log2 units
-constexpr float kSumMin = 0x1p-48f, kSumMax = 0x1p+64f;     // row sums a tile without running maxima is accepted with
 constexpr float kFreshFloor = -4.0f;            // a row's first scores are taken against 0 if their max is in [-4, 8]
 enum Bar : int {
   BAR_Q_FULL = 0,                                  // 2: Q tile of a query block landed
@@ -104,8 +92,7 @@ struct Smem {
   static constexpr uint32_t off_bits = off_v + kStagesV * kTileBytes;      // [kBitStages][4 sub-slots][128 rows] u32
   static constexpr uint32_t off_bar = off_bits + kBitStages * 4 * 128 * 4;
   static constexpr uint32_t off_misc = off_bar + 8 * 48;
-  static constexpr uint32_t off_done = off_misc + 16 + 16 * kTileRing; // misc: TMEM base, abort flag, tile ring (index, the two list lengths, whether to be careful)
-  static constexpr uint32_t off_ids = off_done + 16 * kDoneRing;       // done ring: tile index, the two list lengths, whether it has to be done again
+  static constexpr uint32_t off_ids = off_misc + 16 + 16 * kTileRing;  // misc: TMEM base, abort flag, tile ring (index and the two list lengths per slot)
   static constexpr uint32_t off_xch = off_ids + 2 * 4 * 4 * 4;         // ids: per producer warp [4 steps][4 entries]; xch: [2 parities + epilogue][kSplit column groups][128 rows] f32
   static constexpr uint32_t total = off_xch + 3 * kSplit * 128 * 4;
   static constexpr uint32_t dynamic_bytes = total + 1024;       // slack to align the base to 1024 B
@@ -114,7 +101,6 @@ static_assert(BAR_COUNT <= 48, "barrier area too small");
 
 template <typename T> struct Fmt;
 template <> struct Fmt<__half> {
-  static constexpr bool wide_range = false;          // P must stay within a few powers of two of 1
   static constexpr uint32_t umma = 0;
   static __device__ __forceinline__ uint32_t pack2(float a, float b) {
     __half2 h = __floats2half2_rn(a, b);
@@ -122,7 +108,6 @@ template <> struct Fmt<__half> {
   }
 };
 template <> struct Fmt<__nv_bfloat16> {
-  static constexpr bool wide_range = true;           // the exponent range of fp32: P keeps its precision at any size
   static constexpr uint32_t umma = 1;
   static __device__ __forceinline__ uint32_t pack2(float a, float b) {
     __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
@@ -204,59 +189,6 @@ __device__ __forceinline__ void softmax_pass(uint32_t t_s, uint32_t t_p, float s
   ptx::unpack_f32x2(sum2[0], s0, s1);
   sum_out = s0 + s1;
   xmax_out = xmax[0];
-}
-
-// The pass without a reference (types with the exponent range of fp32): P = exp2(s*scale), no maximum.
-template <typename T, bool kMasked>
-__device__ __forceinline__ void plain_chunk(const uint32_t (&r)[32], uint32_t w, uint64_t scale2, uint32_t (&pk)[16],
-                                            uint64_t (&sum2v)[kAcc]) {
-#pragma unroll
-  for (int i = 0; i < 16; ++i) {
-    float x0, x1;
-    ptx::unpack_f32x2(ptx::mul_f32x2(ptx::pack_u32x2(r[2 * i], r[2 * i + 1]), scale2), x0, x1);
-    if (kMasked) {
-      x0 = (w >> (2 * i)) & 1u ? x0 : -INFINITY;                 // line 47
-      x1 = (w >> (2 * i + 1)) & 1u ? x1 : -INFINITY;
-    }
-    const float p0 = ex2_approx(x0), p1 = ex2_approx(x1);
-    sum2v[i % kAcc] = ptx::add_f32x2(sum2v[i % kAcc], ptx::pack_f32x2(p0, p1));
-    pk[i] = Fmt<T>::pack2(p0, p1);
-  }
-}
-template <typename T, bool kMasked, int kCW>
-__device__ __forceinline__ float plain_pass(uint32_t t_s, uint32_t t_p, uint64_t scale2, const uint32_t (&w)[kCW / 32]) {
-  constexpr int kChunks = kCW / 32;
-  uint32_t r[kChunks][32];
-#pragma unroll
-  for (int c = 0; c < kChunks; ++c) ptx::tmem_ld32(t_s + 32 * c, r[c]);
-  bool dead[kChunks], solid[kChunks];
-#pragma unroll
-  for (int c = 0; c < kChunks; ++c) {
-    dead[c] = kMasked && __all_sync(0xffffffffu, w[c] == 0u);
-    solid[c] = !kMasked || __all_sync(0xffffffffu, w[c] == 0xffffffffu);
-  }
-  ptx::tmem_ld_wait();
-  uint64_t sum2[kAcc];
-#pragma unroll
-  for (int a = 0; a < kAcc; ++a) sum2[a] = ptx::pack_f32x2(0.f, 0.f);
-#pragma unroll
-  for (int c = 0; c < kChunks; ++c) {
-    uint32_t pk[16];
-    if (dead[c]) {
-#pragma unroll
-      for (int i = 0; i < 16; ++i) pk[i] = 0u;
-    } else if (solid[c]) {
-      plain_chunk<T, false>(r[c], w[c], scale2, pk, sum2);
-    } else {
-      plain_chunk<T, true>(r[c], w[c], scale2, pk, sum2);
-    }
-    ptx::tmem_st16(t_p + 16 * c, pk);
-  }
-#pragma unroll
-  for (int a = 1; a < kAcc; ++a) sum2[0] = ptx::add_f32x2(sum2[0], sum2[a]);
-  float s0, s1;
-  ptx::unpack_f32x2(sum2[0], s0, s1);
-  return s0 + s1;
 }
 
 // Moves kCols fp32 columns between tensor memory and registers (kCols = 32 or 16).
@@ -366,13 +298,11 @@ attn_fwd_tc_kernel(const __grid_constant__ AttnParams p,
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + L::off_misc);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + L::off_misc + 4);
   volatile int* tile_ring = reinterpret_cast<volatile int*>(smem + L::off_misc + 16);
-  volatile int* done_ring = reinterpret_cast<volatile int*>(smem + L::off_done);
   float* xch = reinterpret_cast<float*>(smem + L::off_xch);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // The epilogue stages a tile of O in the Q slot it has finished with and stores it with TMA when a
   // thread's share of a row is one 128-byte swizzle row; otherwise the threads store their rows directly.
-  constexpr bool kOptimistic = Fmt<T>::wide_range;
   constexpr bool kStageO = (D / kSplit) * sizeof(T) == 128;
   const int nq = (p.Sq + kTileM - 1) / kTileM;
   const int nk = p.Sk / p.BK;
@@ -408,7 +338,6 @@ attn_fwd_tc_kernel(const __grid_constant__ AttnParams p,
       ptx::mbar_init(bar(BAR_TILE_FULL + i), 1);
       ptx::mbar_init(bar(BAR_TILE_EMPTY + i), 3 + 4 * kSplit);    // V producer, two issuers, softmax warps
     }
-    for (int i = 0; i < kDoneRing; ++i) done_ring[4 * i + 3] = 0;
     *abort_flag = 0;
     ptx::fence_mbar_init();
   }
@@ -434,14 +363,12 @@ attn_fwd_tc_kernel(const __grid_constant__ AttnParams p,
   // decision as a whole, so that no lane is left alone in a warp-wide tensor-memory instruction.
   // Whole warps wait, also where one lane acts on the result: a lone lane polling a barrier (the other
   // lanes parked at the reconvergence point) notices its completion several times later than a full warp.
-  bool careful = false;                            // of the tile next_tile_warp returned last: with the running maximum
   auto next_tile_warp = [&](int ord, int& n_full, int& n_part) -> int {
     const int slot = ord % kTileRing;
     if (!__all_sync(0xffffffffu, ptx::mbar_wait(bar(BAR_TILE_FULL + slot), (ord / kTileRing) & 1, abort_flag))) return n_tiles;
     const int t = tile_ring[4 * slot];
     n_full = tile_ring[4 * slot + 1];
     n_part = tile_ring[4 * slot + 2];
-    careful = tile_ring[4 * slot + 3] != 0;
     __syncwarp();
     if (lane == 0) ptx::mbar_arrive(bar(BAR_TILE_EMPTY + slot));
     return t;
@@ -469,51 +396,14 @@ attn_fwd_tc_kernel(const __grid_constant__ AttnParams p,
     int st = 0, round = 0, gu = 0, tq = 0;
     const uint32_t s_ids = sbase + L::off_ids + static_cast<uint32_t>(warp) * 64u;
     const volatile int* ids_ring = reinterpret_cast<const volatile int*>(smem + L::off_ids + warp * 64);
-    // lane 0 of warp 0 publishes tile `t`, with its two list lengths, as ordinal `ord` of the sequence -- or, in its
-    // place, a tile that the softmax gave up for a second, careful try; `t` is then held back for the next turn.  A
-    // role that has read ordinal x is through with those before it, so the outcome of a tile is known when the ordinal
-    // behind it has been read by every role: no signal of its own.  Before the end of the sequence comes a turn
-    // without a tile (-1) for that.
-    int held = -1, done_ord = 0, known_ord = 0, pause_ord = -1;   // outcomes looked at; known (of ordinals below)
-    auto publish = [&](int ord, int& t, int& n_full, int& n_part) {
+    // lane 0 of warp 0 publishes tile `t`, with its two list lengths, as ordinal `ord` of the sequence
+    auto publish = [&](int ord, int t, int n_full, int n_part) {
       const int slot = ord % kTileRing;
       if (ord >= kTileRing) ok = ptx::mbar_wait(bar(BAR_TILE_EMPTY + slot), (ord / kTileRing - 1) & 1, abort_flag);
-      int careful_try = 0;
-      if (kOptimistic) {
-        held = -1;
-        known_ord = max(known_ord, ord - kTileRing);            // every role has read ordinal ord - kTileRing
-        if (pause_ord >= known_ord) {
-          if (ok) ok = ptx::mbar_wait(bar(BAR_TILE_EMPTY + pause_ord % kTileRing), (pause_ord / kTileRing) & 1, abort_flag);
-          known_ord = pause_ord;
-        }
-        int again = -1;
-        while (ok && again < 0 && done_ord < known_ord) {
-          const int d = done_ord++ % kDoneRing;
-          if (done_ring[4 * d + 3] != 0) {
-            done_ring[4 * d + 3] = 0;
-            again = d;
-          }
-        }
-        if (again >= 0) {
-          held = t;
-          t = done_ring[4 * again]; n_full = done_ring[4 * again + 1]; n_part = done_ring[4 * again + 2];
-          careful_try = 1;
-        } else if (ok && t >= n_tiles && pause_ord < 0) {       // (careful tiles behind it are not judged)
-          held = t;
-          t = -1;
-          pause_ord = ord;
-        }
-      }
       tile_ring[4 * slot] = (ok && *abort_flag == 0) ? t : n_tiles;    // after a failed wait every role is sent home
       tile_ring[4 * slot + 1] = n_full;
       tile_ring[4 * slot + 2] = n_part;
-      tile_ring[4 * slot + 3] = careful_try;
       ptx::mbar_arrive(bar(BAR_TILE_FULL + slot));
-      if (kOptimistic) {                            // (behind the publication, which the other roles wait for)
-        done_ring[4 * (ord % kDoneRing)] = t;
-        done_ring[4 * (ord % kDoneRing) + 1] = n_full;
-        done_ring[4 * (ord % kDoneRing) + 2] = n_part;
-      }
     };
     int ord = 0;
     int tile = blockIdx.x, len_f = 0, len_p = 0;
@@ -532,9 +422,8 @@ attn_fwd_tc_kernel(const __grid_constant__ AttnParams p,
       // the atomic is not waited for until then.
       int drawn = 0;
       if (is_k && lane == 0)
-        drawn = held >= 0 ? held : p.tile_counter != nullptr ? atomicAdd(p.tile_counter, 1) + static_cast<int>(gridDim.x)
+        drawn = p.tile_counter != nullptr ? atomicAdd(p.tile_counter, 1) + static_cast<int>(gridDim.x)
                                           : tile + static_cast<int>(gridDim.x);
-      if (tile >= 0) {
       const TileInfo ti = tile_info(p, tile, len_f, len_p, nq, nk, eps_shift);
       const int b = ti.b, h = ti.h, qblk = ti.qblk, n_full = ti.n_full, total = ti.total, n_steps = ti.n_steps,
                 n_plain = ti.n_plain, j0 = ti.j0, j1 = ti.j1;
@@ -623,7 +512,6 @@ attn_fwd_tc_kernel(const __grid_constant__ AttnParams p,
       gu += max(j1 - ti.m0, 0);
       ++tq;
       }
-      }
       ++ord;
       if (is_k) {
         if (lane == 0) {
@@ -658,7 +546,6 @@ attn_fwd_tc_kernel(const __grid_constant__ AttnParams p,
         int len_f, len_p;
         const int tile = next_tile_warp(ord, len_f, len_p);
         if (tile >= n_tiles) break;
-        if (tile < 0) continue;
         const TileInfo ti = tile_info(p, tile, len_f, len_p, nq, nk, eps_shift);
         if (ti.n_steps == 0) continue;
         const int qs = tq & 1;
@@ -705,7 +592,6 @@ attn_fwd_tc_kernel(const __grid_constant__ AttnParams p,
         int len_f, len_p;
         const int tile = next_tile_warp(ord, len_f, len_p);
         if (tile >= n_tiles) break;
-        if (tile < 0) continue;
         const TileInfo ti = tile_info(p, tile, len_f, len_p, nq, nk, eps_shift);
         if (ti.n_steps == 0) continue;
         for (int j = 0; j < ti.n_steps && ok; ++j, ++g) {
@@ -754,7 +640,6 @@ attn_fwd_tc_kernel(const __grid_constant__ AttnParams p,
     const uint32_t lane_off = static_cast<uint32_t>(lq * 32) << 16;
     const uint32_t tO_mine = tO + lane_off + kOC * quarter;
     const float scale = p.scale_log2;
-    const uint64_t scale2 = ptx::pack_f32x2(scale, scale);
     int g0 = 0, gu = 0, tq = 0;
     int stored_slot = -1;                          // Q slot holding a staged O tile whose store is in flight
     if (kStageO && warp == kSoftmaxWarp0 && lane == 0) ptx::prefetch_tensormap(&tm_o);
@@ -773,7 +658,6 @@ attn_fwd_tc_kernel(const __grid_constant__ AttnParams p,
       int len_f, len_p;
       const int tile = next_tile_warp(ord, len_f, len_p);
       if (tile >= n_tiles) break;
-      if (tile < 0) { release_staged(); continue; }
       const TileInfo ti = tile_info(p, tile, len_f, len_p, nq, nk, eps_shift);
       const int n_full = ti.n_full, total = ti.total, n_steps = ti.n_steps, n_plain = ti.n_plain;
       release_staged();
@@ -785,18 +669,14 @@ attn_fwd_tc_kernel(const __grid_constant__ AttnParams p,
       // The 32 rows of this warp exist (a short last query block has none for some warps: those do no arithmetic
       // and write nothing).
       const bool rows_live = ti.qblk * kTileM + lq * 32 < p.Sq;
+      if (n_steps == 0 && !rows_live) continue;
       if (n_steps == 0) {                          // nothing attended (in this range): the rows are 0
-        if (rows_live) {
 #pragma unroll
-          for (int i = 0; i < kOC / 8; ++i) dst[i] = make_uint4(0u, 0u, 0u, 0u);
-          if (lse_row != nullptr && quarter == 0) *lse_row = -INFINITY;
-        }
+        for (int i = 0; i < kOC / 8; ++i) dst[i] = make_uint4(0u, 0u, 0u, 0u);
+        if (lse_row != nullptr && quarter == 0) *lse_row = -INFINITY;
         continue;
       }
-      const int mask_from = rows_live ? n_plain : ti.j0;            // first step with mask work for this warp
-      const bool plain = kOptimistic && !careful;  // no reference: P = exp2(x), judged by the row sums at the end
-      float m = plain ? 0.f : -INFINITY, l = 0.f;  // lines 103-104; l holds this group's partial sum
-      uint32_t seen = 0;                           // non-zero once this thread had a column it attends (plain)
+      float m = -INFINITY, l = 0.f;                // lines 103-104; l holds this group's partial sum
       bool gave_up = false;
       for (int jj = 0; jj < n_steps; ++jj) {
         const int j = ti.j0 + jj;                  // step of the walk over the lists
@@ -825,42 +705,25 @@ attn_fwd_tc_kernel(const __grid_constant__ AttnParams p,
         // this group's scores of buffer g & 1, and where its P goes
         const uint32_t tS_mine = tmem_base + 128u * (g & 1) + lane_off + kCW * quarter;
         const uint32_t tP_mine = tmem_base + 384u + 64u * (g & 1) + lane_off + (kCW / 2) * quarter;
-        const bool masked = j >= mask_from;
+        const bool masked = j >= n_plain;
         uint32_t w[kCW / 32];
 #pragma unroll
         for (int c = 0; c < kCW / 32; ++c) w[c] = 0xffffffffu;
         if (masked) {
-          if (j >= n_plain) {
-            const int u = gu + (j - ti.m0), st = u % kBitStages;
+          const int u = gu + (j - ti.m0), st = u % kBitStages;
 #pragma unroll
-            for (int c = 0; c < kCW / 32; ++c) {
-              const int ss = quarter * (kCW / 32) + c;           // sub-slot of the step
-              const int e = (j << eps_shift) + (ss >> sps_shift);
-              const uint32_t word = bits_smem[(st * 4 + ss) * 128 + row];    // stale for a full or padding slot
-              w[c] = e < n_full ? 0xffffffffu : (e < total ? word : 0u);
-            }
-            __syncwarp();
-            if (lane == 0) ptx::mbar_arrive(bar(BAR_BITS_EMPTY + st));
+          for (int c = 0; c < kCW / 32; ++c) {
+            const int ss = quarter * (kCW / 32) + c;           // sub-slot of the step
+            const int e = (j << eps_shift) + (ss >> sps_shift);
+            const uint32_t word = bits_smem[(st * 4 + ss) * 128 + row];    // stale for a full or padding slot
+            w[c] = e < n_full ? 0xffffffffu : (e < total ? word : 0u);
           }
-          if (!rows_live) {
-#pragma unroll
-            for (int c = 0; c < kCW / 32; ++c) w[c] = 0u;
-          }
-        }
-        if (plain) {
-          if (masked) {
-#pragma unroll
-            for (int c = 0; c < kCW / 32; ++c) seen |= w[c];
-            l += plain_pass<T, true, kCW>(tS_mine, tP_mine, scale2, w);
-          } else {
-            seen = 1u;
-            l += plain_pass<T, false, kCW>(tS_mine, tP_mine, scale2, w);
-          }
-          ptx::tmem_st_wait();
-          ptx::tc_fence_before();
           __syncwarp();
-          if (lane == 0) ptx::mbar_arrive(bar(BAR_P_FULL + (g & 1)));
-          continue;
+          if (lane == 0) ptx::mbar_arrive(bar(BAR_BITS_EMPTY + st));
+        }
+        if (!rows_live) {
+#pragma unroll
+          for (int c = 0; c < kCW / 32; ++c) w[c] = 0u;
         }
         float* xch_mine = xch + ((g & 1) * kSplit + quarter) * 128 + row;
         const float* xch_row = xch + (g & 1) * kSplit * 128 + row;
@@ -882,7 +745,7 @@ attn_fwd_tc_kernel(const __grid_constant__ AttnParams p,
         bool second_pass = true;
         {
           float sum, xmax;
-          if (masked) softmax_pass<T, true, kCW>(tS_mine, tP_mine, scale, m_try, w, sum, xmax);
+          if (masked || !rows_live) softmax_pass<T, true, kCW>(tS_mine, tP_mine, scale, m_try, w, sum, xmax);
           else        softmax_pass<T, false, kCW>(tS_mine, tP_mine, scale, m_try, w, sum, xmax);
           *xch_mine = xmax;
           ptx::named_bar_sync(1 + lq, 32 * kSplit);
@@ -925,8 +788,7 @@ attn_fwd_tc_kernel(const __grid_constant__ AttnParams p,
       }
       ptx::tc_fence_after();
       float* xl = xch + 2 * kSplit * 128;
-      // (a sum of 0 over attended columns has underflowed: not a row without any)
-      xl[quarter * 128 + row] = plain && l == 0.f && seen != 0u ? __int_as_float(0x7fffffff) : l;
+      xl[quarter * 128 + row] = l;
       ptx::named_bar_sync(1 + lq, 32 * kSplit);
       if (*abort_flag != 0) break;                 // the other warp of these rows gave up and only arrived
       float l_row = xl[row];
@@ -945,18 +807,6 @@ attn_fwd_tc_kernel(const __grid_constant__ AttnParams p,
         for (int i = 0; i < kOChunk; ++i) ro[c * kOChunk + i] = r[i];
       }
       ptx::tc_fence_before();
-      if (plain) {
-        // Every row sum lies where neither it nor a product with V has lost anything, and no accumulator has
-        // overflowed: else the tile comes again, with running maxima (0 * x is 0 for a finite x only).
-        uint64_t zero2 = ptx::pack_f32x2(0.f, 0.f);
-        const uint64_t by0 = zero2;
-#pragma unroll
-        for (int i = 0; i < kOC / 2; ++i) zero2 = ptx::fma_f32x2(ptx::pack_u32x2(ro[2 * i], ro[2 * i + 1]), by0, zero2);
-        float z0, z1;
-        ptx::unpack_f32x2(zero2, z0, z1);
-        const bool good = z0 == 0.f && z1 == 0.f && (l_row == 0.f || (l_row >= kSumMin && l_row <= kSumMax));
-        if (__any_sync(0xffffffffu, rows_live && !good) && lane == 0) done_ring[4 * (ord % kDoneRing) + 3] = 1;
-      }
       __syncwarp();
       if (lane == 0) ptx::mbar_arrive(bar(BAR_O_FREE));             // O may be overwritten by the next tile
       // A wait that ran out leaves the abort flag set; nothing is written in that case.
@@ -978,7 +828,6 @@ attn_fwd_tc_kernel(const __grid_constant__ AttnParams p,
         ptx::fence_proxy_async();
         __syncwarp();
         if (lane == 0 && live) {
-          if (kOptimistic && careful) ptx::bulk_wait_group0();      // the first try's store of these rows is behind us
           ptx::tma_store_4d(&tm_o, slab, kOC * quarter, ti.qblk * kTileM + lq * 32, p.os[1] ? ti.h : 0,
                             p.os[0] ? ti.b_out : 0);                                  // line 146
           ptx::bulk_commit_group();
