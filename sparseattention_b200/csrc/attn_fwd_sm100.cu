@@ -34,6 +34,8 @@
 // the tensor map fills its missing rows with zeros, the warps of missing rows skip the arithmetic and the stores.
 // Padding Q and the mask to 128 rows in memory instead cost a quarter of such a call: B=8 H=32 Sq=32 Sk=32768,
 // a quarter of the keys, 246 -> 207 us a call; B=3 H=7 S=1120 D=64 with a mask per head 166 -> 41 us (host work included).
+// Such calls run an instantiation of their own (kShort): a check of the rows in every step would cost the others 1 to 3 %
+// (stage 2 of the headline shape at p = 0.5 1875 us with it, 1855 without; B=4 H=32 S=4096 D=64 970 and 940).
 //
 // A step whose last slots run past the end of the lists re-loads the first listed block with an
 // all-zero mask word.  Every mbarrier wait is bounded; on expiry the CTA reports
@@ -43,6 +45,7 @@
 #include <cuda_fp16.h>
 
 #include <mutex>
+#include <type_traits>
 
 #include "ptx_sm100.cuh"
 #include "sa_common.cuh"
@@ -279,7 +282,7 @@ __device__ __noinline__ TileInfo tile_info(const AttnParams& p, int tile, int n_
   return t;
 }
 
-template <typename T, int D>
+template <typename T, int D, bool kShort>
 __global__ void __launch_bounds__(kThreadsTC, 1)
 attn_fwd_tc_kernel(const __grid_constant__ AttnParams p,
                    const __grid_constant__ CUtensorMap tm_q,
@@ -304,7 +307,7 @@ attn_fwd_tc_kernel(const __grid_constant__ AttnParams p,
   // The epilogue stages a tile of O in the Q slot it has finished with and stores it with TMA when a
   // thread's share of a row is one 128-byte swizzle row; otherwise the threads store their rows directly.
   constexpr bool kStageO = (D / kSplit) * sizeof(T) == 128;
-  const int nq = (p.Sq + kTileM - 1) / kTileM;
+  const int nq = kShort ? (p.Sq + kTileM - 1) / kTileM : p.Sq / kTileM;
   const int nk = p.Sk / p.BK;
   // BLOCK_K is 32, 64 or 128: list entries per step (4, 2, 1) and 32-column sub-slots per entry
   // (1, 2, 4) are powers of two, so the per-step index arithmetic is shifts.
@@ -668,7 +671,7 @@ attn_fwd_tc_kernel(const __grid_constant__ AttnParams p,
           : p.lse + (static_cast<int64_t>(ti.b_out) * p.H + ti.h) * p.Sq + ti.qblk * kTileM + row;
       // The 32 rows of this warp exist (a short last query block has none for some warps: those do no arithmetic
       // and write nothing).
-      const bool rows_live = ti.qblk * kTileM + lq * 32 < p.Sq;
+      const bool rows_live = !kShort || ti.qblk * kTileM + lq * 32 < p.Sq;
       if (n_steps == 0 && !rows_live) continue;
       if (n_steps == 0) {                          // nothing attended (in this range): the rows are 0
 #pragma unroll
@@ -918,10 +921,10 @@ bool tma_friendly(const void* base, const int64_t* st) {
 
 namespace {
 
-template <typename T, int D>
+template <typename T, int D, bool kShort>
 int launch_inst(const AttnParams& p, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv,
                 const CUtensorMap& mo, cudaStream_t stream) {
-  auto kernel = attn_fwd_tc_kernel<T, D>;
+  auto kernel = attn_fwd_tc_kernel<T, D, kShort>;
   const DeviceInfo* info = current_device_info();
   if (info == nullptr) return SA_ERR_NO_DEVICE;
   // the opt-in to this much dynamic shared memory is per device and instantiation: done once each
@@ -1023,12 +1026,16 @@ int launch_attn_tc(const AttnParams& p_in, cudaStream_t stream) {
   if (!make_map(&mk, p.k, p.dtype, p.B, p.H, p.Sk, p.D, p.ks, p.BK)) return SA_ERR_CUDA;
   if (!make_map(&mv, p.v, p.dtype, p.B, p.H, p.Sk, p.D, p.vs, p.BK)) return SA_ERR_CUDA;
   if (!make_map(&mo, p.o, p.dtype, p.B * p.splits, p.H, p.Sq, p.D, p.os, 32)) return SA_ERR_CUDA;     // one softmax warp's rows
-  if (p.dtype == SA_DTYPE_BF16) {
-    return p.D == 128 ? launch_inst<__nv_bfloat16, 128>(p, mq, mk, mv, mo, stream)
-                      : launch_inst<__nv_bfloat16, 64>(p, mq, mk, mv, mo, stream);
-  }
-  return p.D == 128 ? launch_inst<__half, 128>(p, mq, mk, mv, mo, stream)
-                    : launch_inst<__half, 64>(p, mq, mk, mv, mo, stream);
+  auto launch = [&](auto type, auto width) {
+    using T = decltype(type);
+    constexpr int D = decltype(width)::value;
+    return p.Sq % kTileM != 0 ? launch_inst<T, D, true>(p, mq, mk, mv, mo, stream)
+                              : launch_inst<T, D, false>(p, mq, mk, mv, mo, stream);
+  };
+  using D64 = std::integral_constant<int, 64>;
+  using D128 = std::integral_constant<int, 128>;
+  if (p.dtype == SA_DTYPE_BF16) return p.D == 128 ? launch(__nv_bfloat16(), D128()) : launch(__nv_bfloat16(), D64());
+  return p.D == 128 ? launch(__half(), D128()) : launch(__half(), D64());
 }
 
 }  // namespace sa
