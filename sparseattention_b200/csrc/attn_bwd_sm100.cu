@@ -356,6 +356,9 @@ __device__ __forceinline__ void bwd_body(const BwdArgs& a, const CUtensorMap* tm
     auto issue_s = [&](int j) {
       const int st = j & 1;
       if (!wait(BB_X_FULL + st, j >> 1)) return;
+      // Products with different accumulators are not promised to run in the order they are issued: in mode 1 the one
+      // that reads P(j - 1) has to be through before these scores overwrite it.
+      if (MODE == 1 && j > 0 && !wait(BB_Y_EMPTY + (st ^ 1), (j - 1) >> 1)) return;
       ptx::tc_fence_after();
       if (lane == 0) {
         product(kColS, a1_lo, x_lo + st * kStageStep);
@@ -366,6 +369,8 @@ __device__ __forceinline__ void bwd_body(const BwdArgs& a, const CUtensorMap* tm
     auto issue_t = [&](int j) {
       const int st = j & 1;
       if (!wait(BB_Y_FULL + st, j >> 1)) return;
+      // (dS(j - 1) likewise; mode 0 has two buffers, and dS(j - 2) was read before X(j) could be loaded)
+      if (MODE == 1 && j > 0 && !wait(BB_X_EMPTY + (st ^ 1), (j - 1) >> 1)) return;
       ptx::tc_fence_after();
       if (lane == 0) {
         product(MODE == 0 ? kColT + 128u * st : kColT, a2_lo, y_lo + st * kStageStep);
@@ -388,8 +393,6 @@ __device__ __forceinline__ void bwd_body(const BwdArgs& a, const CUtensorMap* tm
         }
         __syncwarp();
       }
-      // The products of one thread run in the order they are issued: the scores of the next step may overwrite
-      // P once the product that reads it is in front of them.
       if (j + 1 < n_steps) issue_s(j + 1);
       if (MODE == 0 && ok && j + 1 < n_steps) issue_t(j + 1);            // into the other T buffer
       if (!ok || !wait(BB_DS_FULL + st, j >> 1)) break;

@@ -63,6 +63,28 @@ def test_gradients_at_the_edges_of_the_tiles(native_lib, kind, B, H, Sq, Sk, D, 
         _check(leaf.grad, torch.nan_to_num(ref), f"{name} {kind} Sq={Sq} Sk={Sk} D={D} bk={bk}")
 
 
+@pytest.mark.parametrize("Sq,Sk,D,dtype", [(4096, 256, 128, torch.bfloat16), (256, 4096, 64, torch.float16)])
+def test_long_walks(native_lib, Sq, Sk, D, dtype):
+    """32 steps that reuse the same columns of tensor memory for the scores, P, the other product and dS: any step that
+    overwrote them early would show against the generic backward, or from one run to the next."""
+    B, H = 3, 17                                               # 1734 tiles: every SM has several
+    q, k, v, w = (t.to(DEV) for t in _inputs(B, H, Sq, Sk, D, dtype, seed=D))
+    mask = _mask("ragged", B, 1, Sq, Sk, seed=D).to(DEV) | torch.rand((B, 1, Sq // 128, Sk // 128), device=DEV).lt(0.7) \
+        .repeat_interleave(128, 2).repeat_interleave(128, 3)
+    mask = mask.expand(B, H, Sq, Sk)
+    md = sa.compute_mask_kernel(mask, 128, 32)
+    lists = (md.unmasked_kv_ids, md.unmasked_lens, md.masked_kv_ids, md.masked_lens)
+    o, lse = _native.attn_fwd_op(q, k, v, mask, md.packed_bits, *lists, 128, 32, _native.SA_IMPL_AUTO, False, True)
+    want = _native._transposed_and_bwd(q, k, v, o, w, lse, None, mask, *lists, 128, 32)
+    first = None
+    for _ in range(4):
+        got = _native.attn_grads_op(q, k, v, o, w, lse, None, mask, md.packed_bits, *lists, 128, 32)
+        first = first or got
+        for name, g, r, f in zip(("dq", "dk", "dv"), got, want, first):
+            _check(g, r.float().cpu(), name)
+            assert torch.equal(g, f), f"{name}: not the same twice"
+
+
 @pytest.mark.parametrize("bk,per_head_lists", [(32, False), (64, True), (128, True)])
 def test_caller_lists_that_differ_from_the_mask(native_lib, bk, per_head_lists):
     """Lists a caller has pruned and widened: the kernel follows the lists, as the generic backward does."""
