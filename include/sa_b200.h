@@ -18,7 +18,7 @@
 extern "C" {
 #endif
 
-#define SA_ABI_VERSION 5
+#define SA_ABI_VERSION 6
 
 /* status codes */
 #define SA_OK                     0
@@ -225,10 +225,11 @@ int sa_call_attend(const sa_call* call, void* o, float* lse, void* scratch, size
  * sa_attn_bwd_packed; lse is required, d_lse optional; o, d_o, dq, dk, dv contiguous and 16-byte aligned.  The
  * mask is not read (any 16-byte aligned pointer will do).  SA_ERR_UNSUPPORTED for a call that did not run the
  * tensor-core kernel, or with a short last query block.
- * workspace: sa_attn_bwd_packed_workspace_bytes(B, H, distinct mask planes, Sq, Sk) bytes, 256-byte aligned. */
+ * workspace: sa_attn_bwd_packed_workspace_bytes(B, H, distinct mask planes, Sq, Sk) bytes, 256-byte aligned.
+ * dev_status as in sa_attn_fwd: a tile whose wait ran out writes none of its gradients and says so there only. */
 int sa_call_grad(const sa_call* call, const void* o, const float* lse, const void* scratch, size_t scratch_bytes,
                  const void* d_o, const float* d_lse, void* dq, void* dk, void* dv,
-                 void* workspace, size_t workspace_bytes, void* stream);
+                 void* workspace, size_t workspace_bytes, int32_t* dev_status, void* stream);
 
 /* No counterpart in the reference (its README lists a backward pass as future work, README.md:61-65).
  * kv-major lists from the query-major lists of sa_classify_mask: for every (plane, kv block) the

@@ -19,7 +19,7 @@ _PKG_DIR = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.environ.get("SPARSEATTN_B200_LIB") or os.path.join(_PKG_DIR, "libsparseattn_b200.so")
 
 # mirrors of the header's constants
-SA_ABI_VERSION = 5
+SA_ABI_VERSION = 6
 SA_OK = 0
 SA_ERR_UNSUPPORTED = -2
 SA_DTYPE_F32, SA_DTYPE_F16, SA_DTYPE_BF16 = 0, 1, 2
@@ -57,7 +57,7 @@ SYMBOLS = {
     "sa_call_plan": (_i, [ctypes.c_char_p, _p]),
     "sa_call_run": (_i, [ctypes.c_char_p, _p, _p, _p, _sz, _p, _sz, _p, _p]),
     "sa_call_attend": (_i, [ctypes.c_char_p, _p, _p, _p, _sz, _p, _p]),
-    "sa_call_grad": (_i, [ctypes.c_char_p, _p, _p, _p, _sz, _p, _p, _p, _p, _p, _p, _sz, _p]),
+    "sa_call_grad": (_i, [ctypes.c_char_p, _p, _p, _p, _sz, _p, _p, _p, _p, _p, _p, _sz, _p, _p]),
     "sa_selftest_bounded_wait": (_i, [ctypes.c_uint64, _p, _p, _p]),
     "sa_transpose_lists": (_i, [_p, _p, _p, _p, _i, _i, _i, _p, _p, _p, _p, _p]),
     "sa_attn_bwd_workspace_bytes": (_sz, [_i, _i, _i]),
@@ -445,7 +445,7 @@ class _FusedAttention(torch.autograd.Function):
     def forward(ctx, q, k, v, mask, call, plan, mask_strides, block_q, block_k, check_status):
         out, lse, scratch = run_call(q, k, mask, call, plan, mask_strides, block_k, True, check_status)
         ctx.save_for_backward(q, k, v, out, lse, scratch)
-        ctx.call_args = (mask_strides, block_q, block_k)
+        ctx.call_args = (mask_strides, block_q, block_k, check_status)
         ctx.set_materialize_grads(False)
         return out, lse
 
@@ -453,7 +453,7 @@ class _FusedAttention(torch.autograd.Function):
     @torch.autograd.function.once_differentiable
     def backward(ctx, d_o, d_lse):
         q, k, v, out, lse, scratch = ctx.saved_tensors
-        mask_strides, block_q, block_k = ctx.call_args
+        mask_strides, block_q, block_k, check_status = ctx.call_args
         lib = load_library()
         dev = q.device
         with torch.cuda.device(dev):
@@ -466,6 +466,7 @@ class _FusedAttention(torch.autograd.Function):
             dk = torch.empty((B, H, Sk, D), dtype=q.dtype, device=dev)
             dv = torch.empty((B, H, Sk, D), dtype=q.dtype, device=dev)
             ws = torch.empty((lib.sa_attn_bwd_packed_workspace_bytes(B, H, planes, Sq, Sk),), dtype=torch.uint8, device=dev)
+            status = torch.zeros((1,), dtype=torch.int32, device=dev) if check_status else None
             rc = SA_ERR_UNSUPPORTED
             for attempt in range(2):
                 # (the mask itself is not read again: its place in the arguments holds an aligned address)
@@ -473,7 +474,7 @@ class _FusedAttention(torch.autograd.Function):
                 rc = lib.sa_call_grad(call, out.data_ptr(), lse.data_ptr(), scratch.data_ptr(), scratch.numel(),
                                       d_o.data_ptr(), None if d_lse is None else d_lse.data_ptr(),
                                       dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), ws.data_ptr(), ws.numel(),
-                                      _stream_ptr(dev))
+                                      status.data_ptr() if check_status else None, _stream_ptr(dev))
                 if rc != SA_ERR_UNSUPPORTED:
                     break
                 # a gradient that starts off a 16-byte boundary, or tensors that a saved-tensor hook gave back in
@@ -481,6 +482,8 @@ class _FusedAttention(torch.autograd.Function):
                 q, k, v, out, lse, scratch, d_o = (t.clone(memory_format=torch.contiguous_format)
                                                    for t in (q, k, v, out, lse, scratch, d_o))
         _check(rc, "sa_call_grad")
+        if check_status:
+            _raise_status(status)
         return dq, dk, dv, None, None, None, None, None, None, None
 
 
@@ -521,7 +524,8 @@ def _attn_bwd_impl(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, o: torch.T
                    lse: torch.Tensor, d_lse: Optional[torch.Tensor], mask: torch.Tensor,
                    full_ids: torch.Tensor, full_lens: torch.Tensor, part_ids: torch.Tensor, part_lens: torch.Tensor,
                    t_full_ids: torch.Tensor, t_full_lens: torch.Tensor, t_part_ids: torch.Tensor,
-                   t_part_lens: torch.Tensor, block_q: int, block_k: int) -> Tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
+                   t_part_lens: torch.Tensor, block_q: int, block_k: int,
+                   check_status: bool = False) -> Tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
     """Gradients of :func:`attn_fwd_op` with respect to q, k, v (``sa_attn_bwd``): ``o`` and ``lse`` are the
     forward's outputs, ``d_o`` / ``d_lse`` their incoming gradients, the lists the ones the forward walked and
     their kv-major transposes (all may be expanded views)."""
@@ -539,6 +543,7 @@ def _attn_bwd_impl(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, o: torch.T
         dv = torch.empty((B, H, Sk, D), dtype=q.dtype, device=dev)
         ws_bytes = int(lib.sa_attn_bwd_workspace_bytes(B, H, Sq))
         ws = torch.empty((ws_bytes,), dtype=torch.uint8, device=dev)
+        status = torch.zeros((1,), dtype=torch.int32, device=dev) if check_status else None
         rc = lib.sa_attn_bwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), d_o.data_ptr(),
                              lse.data_ptr(), None if gl is None else gl.data_ptr(),
                              dq.data_ptr(), dk.data_ptr(), dv.data_ptr(),
@@ -550,8 +555,11 @@ def _attn_bwd_impl(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, o: torch.T
                              part_ids.data_ptr(), _strides(part_ids), part_lens.data_ptr(), _strides(part_lens),
                              t_full_ids.data_ptr(), _strides(t_full_ids), t_full_lens.data_ptr(), _strides(t_full_lens),
                              t_part_ids.data_ptr(), _strides(t_part_ids), t_part_lens.data_ptr(), _strides(t_part_lens),
-                             scale_log2, ws.data_ptr(), ws_bytes, None, _stream_ptr(dev))
+                             scale_log2, ws.data_ptr(), ws_bytes, status.data_ptr() if check_status else None,
+                             _stream_ptr(dev))
     _check(rc, "sa_attn_bwd")
+    if check_status:
+        _raise_status(status)
     return dq, dk, dv
 
 
@@ -560,11 +568,12 @@ attn_bwd_op = torch.library.custom_op("sparseattention::attn_bwd", mutates_args=
 
 @attn_bwd_op.register_fake
 def _(q, k, v, o, d_o, lse, d_lse, mask, full_ids, full_lens, part_ids, part_lens, t_full_ids, t_full_lens,
-      t_part_ids, t_part_lens, block_q, block_k):
+      t_part_ids, t_part_lens, block_q, block_k, check_status=False):
     return q.new_empty(q.shape), k.new_empty(k.shape), v.new_empty(v.shape)
 
 
-def _transposed_and_bwd(q, k, v, o, d_o, lse, d_lse, mask, full_ids, full_lens, part_ids, part_lens, block_q, block_k):
+def _transposed_and_bwd(q, k, v, o, d_o, lse, d_lse, mask, full_ids, full_lens, part_ids, part_lens, block_q, block_k,
+                        check_status=False):
     """The backward over the mask bytes: kv-major lists, then :func:`_attn_bwd_impl`."""
     B, H = q.shape[0], q.shape[1]
     # kv-major lists, built over the distinct planes of the (possibly expanded) lists
@@ -574,14 +583,15 @@ def _transposed_and_bwd(q, k, v, o, d_o, lse, d_lse, mask, full_ids, full_lens, 
     t_lists = transpose_lists(*planes)
     ex = lambda t: t.expand(*((B, H) + tuple(t.shape[2:])))
     return _attn_bwd_impl(q, k, v, o, d_o, lse, d_lse, mask, full_ids, full_lens, part_ids, part_lens,
-                          ex(t_lists[0]), ex(t_lists[1]), ex(t_lists[2]), ex(t_lists[3]), block_q, block_k)
+                          ex(t_lists[0]), ex(t_lists[1]), ex(t_lists[2]), ex(t_lists[3]), block_q, block_k, check_status)
 
 
 @torch.library.custom_op("sparseattention::attn_grads", mutates_args=())
 def attn_grads_op(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, o: torch.Tensor, d_o: torch.Tensor,
                   lse: torch.Tensor, d_lse: Optional[torch.Tensor], mask: torch.Tensor, bits: torch.Tensor,
                   full_ids: torch.Tensor, full_lens: torch.Tensor, part_ids: torch.Tensor, part_lens: torch.Tensor,
-                  block_q: int, block_k: int) -> Tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
+                  block_q: int, block_k: int,
+                  check_status: bool = False) -> Tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
     """Gradients of :func:`attn_fwd_op` from its inputs and outputs: on the tcgen05 kernel where it covers the
     call (``sa_attn_bwd_packed``; it reads ``bits`` and makes the kv-major lists itself), else through
     :func:`transpose_lists` and ``sa_attn_bwd``."""
@@ -594,7 +604,7 @@ def attn_grads_op(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, o: torch.Te
     d_lse = None if d_lse is None else d_lse.to(torch.float32).contiguous()
     lists = (full_ids, full_lens, part_ids, part_lens)
     if bits.numel() == 0 or block_q != 128 or D not in (64, 128) or q.dtype == torch.float32:
-        return _transposed_and_bwd(q, k, v, o, d_o, lse, d_lse, mask, *lists, block_q, block_k)
+        return _transposed_and_bwd(q, k, v, o, d_o, lse, d_lse, mask, *lists, block_q, block_k, check_status)
     bsb = bits.stride(0) if bits.shape[0] > 1 else 0
     bsh = bits.stride(1) if bits.shape[1] > 1 else 0
     p0 = B if bsb or (B > 1 and any(t.stride(0) for t in lists)) else 1
@@ -605,6 +615,7 @@ def attn_grads_op(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, o: torch.Te
         dv = torch.empty((B, H, Sk, D), dtype=q.dtype, device=dev)
         ws_bytes = int(lib.sa_attn_bwd_packed_workspace_bytes(B, H, p0 * p1, Sq, Sk))
         ws = torch.empty((ws_bytes,), dtype=torch.uint8, device=dev)
+        status = torch.zeros((1,), dtype=torch.int32, device=dev) if check_status else None
         rc = lib.sa_attn_bwd_packed(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), d_o.data_ptr(),
                                     lse.data_ptr(), None if d_lse is None else d_lse.data_ptr(),
                                     dq.data_ptr(), dk.data_ptr(), dv.data_ptr(),
@@ -614,15 +625,19 @@ def attn_grads_op(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, o: torch.Te
                                     bits.data_ptr(), bsb, bsh, p0, p1,
                                     full_ids.data_ptr(), _strides(full_ids), full_lens.data_ptr(), _strides(full_lens),
                                     part_ids.data_ptr(), _strides(part_ids), part_lens.data_ptr(), _strides(part_lens),
-                                    D ** -0.5 / math.log(2), ws.data_ptr(), ws_bytes, None, _stream_ptr(dev))
+                                    D ** -0.5 / math.log(2), ws.data_ptr(), ws_bytes,
+                                    status.data_ptr() if check_status else None, _stream_ptr(dev))
     if rc == SA_ERR_UNSUPPORTED:
-        return _transposed_and_bwd(q, k, v, o, d_o, lse, d_lse, mask, *lists, block_q, block_k)
+        return _transposed_and_bwd(q, k, v, o, d_o, lse, d_lse, mask, *lists, block_q, block_k, check_status)
     _check(rc, "sa_attn_bwd_packed")
+    if check_status:
+        _raise_status(status)
     return dq, dk, dv
 
 
 @attn_grads_op.register_fake
-def _(q, k, v, o, d_o, lse, d_lse, mask, bits, full_ids, full_lens, part_ids, part_lens, block_q, block_k):
+def _(q, k, v, o, d_o, lse, d_lse, mask, bits, full_ids, full_lens, part_ids, part_lens, block_q, block_k,
+      check_status=False):
     return q.new_empty(q.shape), k.new_empty(k.shape), v.new_empty(v.shape)
 
 
@@ -640,16 +655,16 @@ def _attn_setup_context(ctx, inputs, output):
         raise RuntimeError("the attention op was called without its log-sum-exp output: no backward is possible "
                            "(sparse_attention asks for it whenever an input requires grad)")
     ctx.save_for_backward(q, k, v, o, lse, mask, bits, full_ids, full_lens, part_ids, part_lens)
-    ctx.blocks = (block_q, block_k)
+    ctx.call_args = (block_q, block_k, check_status)
 
 
 def _attn_backward(ctx, grad_o, grad_lse):
     q, k, v, o, lse, mask, bits, full_ids, full_lens, part_ids, part_lens = ctx.saved_tensors
-    block_q, block_k = ctx.blocks
+    block_q, block_k, check_status = ctx.call_args
     if grad_o is None:
         grad_o = torch.zeros_like(o)
     dq, dk, dv = attn_grads_op(q, k, v, o, grad_o, lse, grad_lse, mask, bits, full_ids, full_lens, part_ids, part_lens,
-                               block_q, block_k)
+                               block_q, block_k, check_status)
     return dq, dk, dv, None, None, None, None, None, None, None, None, None, None, None, None
 
 

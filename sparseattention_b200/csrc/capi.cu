@@ -565,7 +565,7 @@ int sa_call_run(const sa_call* c, void* o, float* lse, void* scratch, size_t scr
 
 int sa_call_grad(const sa_call* c, const void* o, const float* lse, const void* scratch, size_t scratch_bytes,
                  const void* d_o, const float* d_lse, void* dq, void* dk, void* dv,
-                 void* workspace, size_t workspace_bytes, void* stream) {
+                 void* workspace, size_t workspace_bytes, int32_t* dev_status, void* stream) {
   sa::AttnBwdParams p;
   std::memset(&p, 0, sizeof(p));
   CallLayout l;
@@ -579,6 +579,7 @@ int sa_call_grad(const sa_call* c, const void* o, const float* lse, const void* 
   p.fwd.o = const_cast<void*>(o);
   p.fwd.lse = const_cast<float*>(lse);
   p.fwd.scale_log2 = static_cast<float>(1.0 / std::sqrt(static_cast<double>(p.fwd.D)) / std::log(2.0));
+  p.fwd.dev_status = dev_status;
   p.d_o = d_o; p.d_lse = d_lse;
   p.dq = dq; p.dk = dk; p.dv = dv;
   auto dense = [&](int64_t* st, int S) {

@@ -141,8 +141,8 @@ def sparse_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, mask: to
     ``splits=1`` switches the cutting off.
 
     ``check_status`` (default: the SPARSEATTN_B200_CHECK environment variable) makes the call
-    read the kernel's device status word back, which synchronises; by default the call is
-    asynchronous like the reference's.
+    read the kernel's device status word back, which synchronises, and its backward pass likewise; by default
+    both are asynchronous like the reference's call.
     """
     if check_status is None:
         check_status = os.environ.get("SPARSEATTN_B200_CHECK", "0") not in ("", "0")

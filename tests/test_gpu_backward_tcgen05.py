@@ -153,3 +153,35 @@ def test_differentiable_calls_in_the_forms_autograd_has(native_lib):
     twice = torch.autograd.grad(call(), leaves, w, create_graph=True)
     with pytest.raises(RuntimeError):
         torch.autograd.grad(twice[0].sum(), leaves[0])
+
+
+@pytest.mark.parametrize("caller_lists", [False, True])
+def test_a_backward_that_reports_raises(native_lib, caller_lists):
+    """What the backward kernel reports in its status word reaches the caller that asked for it.  A kv-block id outside the
+    tensor (the kernel checks each, and uses block 0) arrives in the saved lists through a saved-tensor hook."""
+    B, H, S, D = 1, 2, 256, 64
+    q, k, v, w = (t.to(DEV) for t in _inputs(B, H, S, S, D, torch.float16, seed=12))
+    mask = torch.ones((B, H, S, S), dtype=torch.bool, device=DEV)
+    leaves = [t.requires_grad_(True) for t in (q, k, v)]
+    md = sa.compute_mask_kernel(mask, 128, 32) if caller_lists else None
+    at = _native.plan_call(q.detach(), k.detach(), v.detach(), mask, 128, 32)[1][5] // 4        # where the full ids start
+
+    def unpack(t):
+        if caller_lists and t.dtype == torch.int32 and tuple(t.shape) == (B, H, S // 128, S // 32):
+            t = t.clone()
+            t[0, 0, 0, 0] = 1 << 20
+        elif t.dtype == torch.uint8:
+            t = t.clone()
+            t.view(torch.int32)[at] = 1 << 20
+        return t
+
+    for check in (True, False):
+        with torch.autograd.graph.saved_tensors_hooks(lambda t: t, unpack):
+            out = sa.sparse_attention(*leaves, mask, 128, 32, mask_metadata=md, check_status=check)
+        if check:
+            with pytest.raises(RuntimeError, match="out of range"):
+                torch.autograd.grad(out, leaves, w)
+        else:
+            torch.autograd.grad(out, leaves, w)
+    out = sa.sparse_attention(*leaves, mask, 128, 32, mask_metadata=md, check_status=True)
+    assert all(torch.isfinite(g).all() for g in torch.autograd.grad(out, leaves, w))
