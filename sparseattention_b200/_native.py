@@ -457,6 +457,8 @@ class _FusedAttention(torch.autograd.Function):
         lib = load_library()
         dev = q.device
         with torch.cuda.device(dev):
+            # (a saved-tensor hook may have given any of these back in another layout; q, k and v go by their strides)
+            out, lse, scratch = out.contiguous(), lse.contiguous(), scratch.contiguous()
             d_o = torch.zeros_like(out) if d_o is None else d_o.contiguous()
             d_lse = None if d_lse is None else d_lse.to(torch.float32).contiguous()
             B, H, Sq, D = q.shape
@@ -605,6 +607,8 @@ def attn_grads_op(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, o: torch.Te
     lists = (full_ids, full_lens, part_ids, part_lens)
     if bits.numel() == 0 or block_q != 128 or D not in (64, 128) or q.dtype == torch.float32:
         return _transposed_and_bwd(q, k, v, o, d_o, lse, d_lse, mask, *lists, block_q, block_k, check_status)
+    if bits.stride(3) != 1 or bits.stride(2) != bits.shape[3]:       # from a saved-tensor hook: planes go by address
+        bits = bits.contiguous()
     bsb = bits.stride(0) if bits.shape[0] > 1 else 0
     bsh = bits.stride(1) if bits.shape[1] > 1 else 0
     p0 = B if bsb or (B > 1 and any(t.stride(0) for t in lists)) else 1

@@ -185,3 +185,38 @@ def test_a_backward_that_reports_raises(native_lib, caller_lists):
             torch.autograd.grad(out, leaves, w)
     out = sa.sparse_attention(*leaves, mask, 128, 32, mask_metadata=md, check_status=True)
     assert all(torch.isfinite(g).all() for g in torch.autograd.grad(out, leaves, w))
+
+
+@pytest.mark.parametrize("caller_lists", [False, True])
+@pytest.mark.parametrize("what", ["lse", "out", "qkv", "lists"])
+def test_saved_tensors_come_back_in_another_layout(native_lib, what, caller_lists):
+    """A saved-tensor hook may hand back any tensor of equal values: transposed in memory, or every second element of a
+    wider buffer.  Same gradients to the bit."""
+    B, H, S, D = 1, 3, 384, 64
+    q, k, v, w = (t.to(DEV) for t in _inputs(B, H, S, S, D, torch.bfloat16, seed=13))
+    mask = _mask("ragged", B, 1, S, S, seed=14).to(DEV)
+    leaves = [t.requires_grad_(True) for t in (q, k, v)]
+    md = sa.compute_mask_kernel(mask.expand(B, H, S, S), 128, 32) if caller_lists else None
+    is_input = lambda t: any(t.data_ptr() == x.data_ptr() for x in leaves)
+    ours = {"lse": lambda t: t.dtype == torch.float32, "out": lambda t: t.dtype == torch.bfloat16 and not is_input(t),
+            "qkv": is_input, "lists": lambda t: t.dtype in (torch.int32, torch.uint8)}[what]
+    changed = []
+
+    def unpack(t):
+        if not ours(t):
+            return t
+        if t.dim() == 1:
+            other = t.new_zeros((t.shape[0], 2))[:, 0].copy_(t)
+        else:
+            dims = (1, 2) if t.dtype == torch.bfloat16 else (-1, -2)          # (heads interleaved: still 16-byte rows)
+            other = t.transpose(*dims).contiguous().transpose(*dims)
+        changed.append(other.stride() != t.stride())
+        return other
+
+    want = torch.autograd.grad(sa.sparse_attention(*leaves, mask, 128, 32, mask_metadata=md), leaves, w)
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: t.detach(), unpack):
+        out = sa.sparse_attention(*leaves, mask, 128, 32, mask_metadata=md)
+    got = torch.autograd.grad(out, leaves, w)
+    assert any(changed)
+    for name, g, r in zip(("dq", "dk", "dv"), got, want):
+        assert torch.equal(g, r), name
