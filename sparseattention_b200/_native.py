@@ -436,10 +436,70 @@ def fused_call(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, mask: torch.Te
     return None if planned is None else run_call(q, k, mask, *planned, block_k, with_lse, check_status)[:2]
 
 
+def _call_grads_impl(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, out: torch.Tensor, lse: torch.Tensor,
+                     scratch: torch.Tensor, d_o: torch.Tensor, d_lse: Optional[torch.Tensor], mask_strides: List[int],
+                     block_q: int, block_k: int, check_status: bool) -> Tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
+    """Gradients of what :func:`run_call` computed, over the lists it left in its scratch (``sa_call_grad``)."""
+    lib = load_library()
+    dev = q.device
+    with torch.cuda.device(dev):
+        # (a saved-tensor hook may have given any of these back in another layout; q, k and v go by their strides)
+        out, lse, scratch = out.contiguous(), lse.contiguous(), scratch.contiguous()
+        d_o = d_o.contiguous()
+        d_lse = None if d_lse is None else d_lse.to(torch.float32).contiguous()
+        B, H, Sq, D = q.shape
+        Sk = k.shape[2]
+        planes = (1 if mask_strides[0] == 0 else B) * (1 if mask_strides[1] == 0 else H)
+        dq = torch.empty((B, H, Sq, D), dtype=q.dtype, device=dev)
+        dk = torch.empty((B, H, Sk, D), dtype=q.dtype, device=dev)
+        dv = torch.empty((B, H, Sk, D), dtype=q.dtype, device=dev)
+        ws = torch.empty((lib.sa_attn_bwd_packed_workspace_bytes(B, H, planes, Sq, Sk),), dtype=torch.uint8, device=dev)
+        status = torch.zeros((1,), dtype=torch.int32, device=dev) if check_status else None
+        rc = SA_ERR_UNSUPPORTED
+        for attempt in range(2):
+            # (the mask itself is not read again: its place in the arguments holds an aligned address)
+            call = _pack_call(q, k, v, scratch.data_ptr(), mask_strides, block_q, block_k, 1)
+            rc = lib.sa_call_grad(call, out.data_ptr(), lse.data_ptr(), scratch.data_ptr(), scratch.numel(),
+                                  d_o.data_ptr(), None if d_lse is None else d_lse.data_ptr(),
+                                  dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), ws.data_ptr(), ws.numel(),
+                                  status.data_ptr() if check_status else None, _stream_ptr(dev))
+            if rc != SA_ERR_UNSUPPORTED:
+                break
+            # a gradient that starts off a 16-byte boundary, or tensors that a saved-tensor hook gave back in
+            # another layout
+            q, k, v, out, lse, scratch, d_o = (t.clone(memory_format=torch.contiguous_format)
+                                               for t in (q, k, v, out, lse, scratch, d_o))
+    _check(rc, "sa_call_grad")
+    if check_status:
+        _raise_status(status)
+    return dq, dk, dv
+
+
+# For a backward that is itself transformed or watched: batched gradients (vmap calls the op once per gradient),
+# dispatch modes, fake tensors.
+call_grads_op = torch.library.custom_op("sparseattention::call_grads", mutates_args=())(_call_grads_impl)
+
+
+@call_grads_op.register_fake
+def _(q, k, v, out, lse, scratch, d_o, d_lse, mask_strides, block_q, block_k, check_status):
+    return q.new_empty(q.shape), k.new_empty(k.shape), v.new_empty(v.shape)
+
+
+def _transformed() -> bool:
+    """Function transforms or dispatch modes are active: what they do to an op they have to see the op for."""
+    return torch._C._are_functorch_transforms_active() or torch._C._len_torch_dispatch_stack() > 0
+
+
+def _bare(t: torch.Tensor) -> bool:
+    """The memory of ``t`` holds its values: no lazy negation, no zeros without storage, no batch of the vmap that
+    ``is_grads_batched`` uses (which is of the plain type, and not a function transform either)."""
+    return not (t.is_neg() or t._is_zerotensor() or torch._C._functorch.is_legacy_batchedtensor(t))
+
+
 class _FusedAttention(torch.autograd.Function):
-    """:func:`run_call` with its gradients (``sa_call_grad``): the backward walks the lists the forward left in its
-    scratch, which is saved with the inputs and outputs.  For eager mode only -- under tracing, function transforms,
-    forward-mode differentiation and dispatch modes the registered ops are used."""
+    """:func:`run_call` with its gradients: the backward walks the lists the forward left in its scratch, which is saved
+    with the inputs and outputs.  The forward is for eager mode only -- under tracing, function transforms, forward-mode
+    differentiation and dispatch modes the registered ops are used."""
 
     @staticmethod
     def forward(ctx, q, k, v, mask, call, plan, mask_strides, block_q, block_k, check_status):
@@ -452,48 +512,18 @@ class _FusedAttention(torch.autograd.Function):
     @staticmethod
     @torch.autograd.function.once_differentiable
     def backward(ctx, d_o, d_lse):
-        q, k, v, out, lse, scratch = ctx.saved_tensors
-        mask_strides, block_q, block_k, check_status = ctx.call_args
-        lib = load_library()
-        dev = q.device
-        with torch.cuda.device(dev):
-            # (a saved-tensor hook may have given any of these back in another layout; q, k and v go by their strides)
-            out, lse, scratch = out.contiguous(), lse.contiguous(), scratch.contiguous()
-            d_o = torch.zeros_like(out) if d_o is None else d_o.contiguous()
-            d_lse = None if d_lse is None else d_lse.to(torch.float32).contiguous()
-            B, H, Sq, D = q.shape
-            Sk = k.shape[2]
-            planes = (1 if mask_strides[0] == 0 else B) * (1 if mask_strides[1] == 0 else H)
-            dq = torch.empty((B, H, Sq, D), dtype=q.dtype, device=dev)
-            dk = torch.empty((B, H, Sk, D), dtype=q.dtype, device=dev)
-            dv = torch.empty((B, H, Sk, D), dtype=q.dtype, device=dev)
-            ws = torch.empty((lib.sa_attn_bwd_packed_workspace_bytes(B, H, planes, Sq, Sk),), dtype=torch.uint8, device=dev)
-            status = torch.zeros((1,), dtype=torch.int32, device=dev) if check_status else None
-            rc = SA_ERR_UNSUPPORTED
-            for attempt in range(2):
-                # (the mask itself is not read again: its place in the arguments holds an aligned address)
-                call = _pack_call(q, k, v, scratch.data_ptr(), mask_strides, block_q, block_k, 1)
-                rc = lib.sa_call_grad(call, out.data_ptr(), lse.data_ptr(), scratch.data_ptr(), scratch.numel(),
-                                      d_o.data_ptr(), None if d_lse is None else d_lse.data_ptr(),
-                                      dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), ws.data_ptr(), ws.numel(),
-                                      status.data_ptr() if check_status else None, _stream_ptr(dev))
-                if rc != SA_ERR_UNSUPPORTED:
-                    break
-                # a gradient that starts off a 16-byte boundary, or tensors that a saved-tensor hook gave back in
-                # another layout
-                q, k, v, out, lse, scratch, d_o = (t.clone(memory_format=torch.contiguous_format)
-                                                   for t in (q, k, v, out, lse, scratch, d_o))
-        _check(rc, "sa_call_grad")
-        if check_status:
-            _raise_status(status)
-        return dq, dk, dv, None, None, None, None, None, None, None
+        saved = ctx.saved_tensors
+        args = (*saved, torch.zeros_like(saved[3]) if d_o is None else d_o, d_lse)
+        eager = _plain(*args[:7]) and not _transformed() and _bare(args[6]) and (d_lse is None or _bare(d_lse))
+        grads = (_call_grads_impl if eager else call_grads_op)(*args, *ctx.call_args)
+        return (*grads, None, None, None, None, None, None, None)
 
 
 def fused_call_with_grad(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, mask: torch.Tensor, block_q: int, block_k: int,
                          check_status: bool):
     """Both stages of a differentiable call: (out, lse), or None for one that is left to the registered ops."""
-    if q.shape[2] % 128 != 0 or torch._C._are_functorch_transforms_active() or torch._C._len_torch_dispatch_stack() > 0 or \
-            torch.autograd.forward_ad._current_level >= 0:
+    if q.shape[2] % 128 != 0 or _transformed() or torch.autograd.forward_ad._current_level >= 0 or \
+            not (_bare(q) and _bare(k) and _bare(v)):
         return None
     planned = plan_call(q, k, v, mask, block_q, block_k)
     if planned is None or planned[1][2] != SA_IMPL_TCGEN05 or k.shape[2] // block_k > 40 * 1024:

@@ -120,6 +120,44 @@ def test_gradient_op_passes_opcheck(native_lib):
     o, lse = _native.attn_fwd_op(q, k, v, mask.expand(B, H, S, S), bits, *lists, 128, 32, _native.SA_IMPL_AUTO, False, True)
     torch.library.opcheck(_native.attn_grads_op, (q, k, v, o, w, lse, torch.ones_like(lse), mask.expand(B, H, S, S), bits,
                                                   *lists, 128, 32), test_utils=("test_schema", "test_faketensor"))
+    call, plan, ms = _native.plan_call(q, k, v, mask, 128, 32)
+    o, lse, scratch = _native.run_call(q, k, mask, call, plan, ms, 32, True, False)
+    torch.library.opcheck(_native.call_grads_op, (q, k, v, o, lse, scratch, w, None, list(ms), 128, 32, False),
+                          test_utils=("test_schema", "test_faketensor"))
+
+
+@pytest.mark.parametrize("caller_lists", [False, True])
+def test_batched_and_watched_gradients(native_lib, caller_lists):
+    """Several gradients at once (``is_grads_batched``, a vectorised Jacobian: vmap over the backward) equal them one by
+    one, and a dispatch mode around the backward sees its op."""
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    class Watch(TorchDispatchMode):
+        seen = []
+
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            self.seen.append(func.namespace)
+            return func(*args, **(kwargs or {}))
+
+    B, H, S, D = 1, 2, 256, 64
+    q, k, v, w = (t.to(DEV) for t in _inputs(B, H, S, S, D, torch.float16, seed=15))
+    mask = workloads.random_block_mask(B, S, 0.5, 0.2, seed=16).to(DEV)
+    leaves = [t.requires_grad_(True) for t in (q, k, v)]
+    md = sa.compute_mask_kernel(mask.expand(B, H, S, S), 128, 32) if caller_lists else None
+    out, lse = sa.sparse_attention(*leaves, mask, 128, 32, mask_metadata=md, return_lse=True)
+    many = torch.stack([w, -w, w.flip(2)])
+    many_lse = torch.randn((3, B, H, S), device=DEV)
+    got = torch.autograd.grad((out, lse), leaves, (many, many_lse), is_grads_batched=True, retain_graph=True)
+    for i in range(3):
+        want = torch.autograd.grad((out, lse), leaves, (many[i], many_lse[i]), retain_graph=True)
+        for name, g, r in zip(("dq", "dk", "dv"), got, want):
+            assert torch.equal(g[i], r), name
+    with Watch() as watch:
+        watched = torch.autograd.grad((out, lse), leaves, (many[i], many_lse[i]))
+    assert "sparseattention" in watch.seen and all(torch.equal(g, r) for g, r in zip(watched, want))
+    row = lambda x: sa.sparse_attention(x, k, v, mask, 128, 32, mask_metadata=md)[0, 0, 7, :2].float()
+    jac = torch.autograd.functional.jacobian(row, q.detach(), vectorize=True)
+    assert torch.equal(jac, torch.autograd.functional.jacobian(row, q.detach())) and jac.abs().max().item() > 0
 
 
 def test_differentiable_calls_in_the_forms_autograd_has(native_lib):
