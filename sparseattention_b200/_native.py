@@ -94,12 +94,12 @@ def load_library():
             f"{LIB_PATH} is missing: build it with `python -m sparseattention_b200.build` "
             "(there is no CPU or PyTorch fallback for these ops)")
     lib = ctypes.CDLL(LIB_PATH)
+    if lib.sa_abi_version() != SA_ABI_VERSION:                 # (before the symbols: another version may lack some)
+        raise NativeLibraryError("libsparseattn_b200.so has a different ABI version; rebuild it")
     for name, (res, args) in SYMBOLS.items():
         fn = getattr(lib, name)
         fn.restype = res
         fn.argtypes = args
-    if lib.sa_abi_version() != SA_ABI_VERSION:
-        raise NativeLibraryError("libsparseattn_b200.so has a different ABI version; rebuild it")
     _lib = lib
     return lib
 

@@ -27,6 +27,17 @@ def test_library_exports_every_declared_symbol(native_lib):
     assert b"unsupported" in native_lib.sa_status_str(-2)
 
 
+def test_a_library_of_another_version_says_so(native_lib, monkeypatch):
+    """An older library lacks newer symbols: the message is about its version, not about the first one missing."""
+    class Old:
+        sa_abi_version = staticmethod(lambda: _native.SA_ABI_VERSION - 1)
+
+    monkeypatch.setattr(_native, "_lib", None)
+    monkeypatch.setattr(_native.ctypes, "CDLL", lambda path: Old())
+    with pytest.raises(_native.NativeLibraryError, match="ABI version"):
+        _native.load_library()
+
+
 def test_argument_validation_needs_no_gpu(native_lib):
     bu, hu = ctypes.c_int(), ctypes.c_int()
     assert native_lib.sa_unique_planes(8, 32, 4096 * 4096, 0, ctypes.byref(bu), ctypes.byref(hu)) == 0
