@@ -132,8 +132,8 @@ def test_backward_op_passes_opcheck(native_lib):
 @pytest.mark.parametrize("dtype,D,bq,bk", [(torch.bfloat16, 128, 64, 64), (torch.float16, 128, 128, 128),
                                           (torch.bfloat16, 64, 32, 32)])
 def test_tensor_core_backward_on_a_mask_with_unaligned_rows(native_lib, dtype, D, bq, bk):
-    """The tensor-core backward kernels with 64 and 32 rows per CTA on either side, and a mask whose rows
-    are not 16-byte aligned (a view into a wider buffer): the mask bytes are then read one by one."""
+    """Plain calls, whose lists are made at 128 rows whatever BLOCK_Q (the tcgen05 backward), under a mask whose rows are
+    not 16-byte aligned (a view into a wider buffer; stage 1 copies it)."""
     B, H, S = 1, 3, 768
     q, k, v = workloads.make_qkv(B, H, S, D, dtype, seed=330 + bq)
     wide = torch.zeros((B, 1, S, S + 8), dtype=torch.bool)
@@ -149,3 +149,29 @@ def test_tensor_core_backward_on_a_mask_with_unaligned_rows(native_lib, dtype, D
         torch.cuda.synchronize()
         for name, got, ref in zip(("dq", "dk", "dv"), (qd.grad, kd.grad, vd.grad), want):
             _assert_grad_close(got, ref, dtype, f"{name} {dtype} D={D} ({bq},{bk}) mask stride {m_dev.stride(2)}")
+
+
+@pytest.mark.parametrize("dtype,D,bq,bk", [(torch.bfloat16, 128, 64, 64), (torch.float16, 128, 32, 128),
+                                          (torch.float16, 64, 64, 32), (torch.bfloat16, 64, 32, 32)])
+def test_warp_level_backward_over_short_caller_lists(native_lib, dtype, D, bq, bk):
+    """Caller lists at 32 and 64 query rows: the warp-level tensor-core backward, with 64 and 32 rows per CTA on either
+    side, over a mask with 16-byte aligned rows and one without (the mask bytes are then read one by one)."""
+    B, H, S = 1, 3, 768
+    q, k, v = workloads.make_qkv(B, H, S, D, dtype, seed=340 + bq)
+    wide = torch.zeros((B, 1, S, S + 8), dtype=torch.bool)
+    wide[..., 4:S + 4] = workloads.document_causal_mask(B, S, (90, 300), 0.15, seed=341 + bk)
+    mask = wide[..., 4:S + 4]
+    g = torch.Generator().manual_seed(10)
+    w = torch.randn((B, H, S, D), generator=g).to(dtype)
+    want = _reference_grads(q, k, v, mask, w)
+    for m_dev in (mask.to(DEV).contiguous(), wide.to(DEV)[..., 4:S + 4]):
+        md = sa.compute_mask_kernel(m_dev.expand(B, H, S, S), bq, bk)
+        leaves = [t.to(DEV).requires_grad_(True) for t in (q, k, v)]
+        out = sa.sparse_attention(*leaves, m_dev, bq, bk, mask_metadata=md, check_status=True)
+        with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+            out.backward(w.to(DEV))
+            torch.cuda.synchronize()
+        ran = {e.key for e in prof.key_averages()}
+        assert any("attn_bwd_mma_kernel" in n for n in ran), ran
+        for name, leaf, ref in zip(("dq", "dk", "dv"), leaves, want):
+            _assert_grad_close(leaf.grad, ref, dtype, f"{name} {dtype} D={D} ({bq},{bk}) mask stride {m_dev.stride(2)}")
