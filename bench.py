@@ -506,7 +506,7 @@ def run_backward(args):
         "forward_ms": fwd_ms, "forward_plus_backward_ms": ours_ms, "backward_ms": ours_ms - fwd_ms,
         "backward_tflops_over_listed_tiles": 2.5 * flops_fwd / ((ours_ms - fwd_ms) * 1e-3) / 1e12,
         "torch_sdpa_bool_mask_forward_plus_backward_ms": sdpa_ms,
-        "note": "backward = kv-major list transpose + dQ and dK/dV kernels on the tensor cores (warp-level MMA, fp32 accumulation); "
+        "note": "backward = row statistics, kv-major lists, then dQ and dK/dV in one launch on tcgen05 (fp32 accumulation); "
                 "2.5 x the forward's FLOPs over the listed tiles",
     }))
 

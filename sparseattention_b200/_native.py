@@ -414,13 +414,16 @@ def run_call(q: torch.Tensor, k: torch.Tensor, mask: torch.Tensor, call: bytes, 
     (scratch_bytes, _, _, _, bq, f_ids, f_lens, p_ids, p_lens, bits, Bu, Hu) = plan
     base = scratch.data_ptr()
     lse_ptr, status_ptr = lse.data_ptr() if with_lse else None, status.data_ptr() if check_status else None
+    # Stage 1 goes through sa_classify_mask, the entry of every other classification, wherever that entry takes the
+    # call; sa_call_run is both stages at once with the short last query block it refuses.  (A call of more tiles than
+    # SMs has a memset of the tile counter between the two kernels in the first form; the classifier clears it in the second.)
     if Sq % bq == 0:
         rc = lib.sa_classify_mask(mask.data_ptr(), *mask_strides, Bu, Hu, Sq, k.shape[2], bq, block_k, base + f_ids,
                                   base + f_lens, base + p_ids, base + p_lens, base + bits if plan[2] == SA_IMPL_TCGEN05 else None,
                                   words.data_ptr(), words.numel(), SA_WS_CLEAN, stream)
         _check(rc, "sa_classify_mask")
         rc = lib.sa_call_attend(call, out.data_ptr(), lse_ptr, base, scratch_bytes, status_ptr, stream)
-    else:                                          # a short last query block: a form only this call makes
+    else:
         rc = lib.sa_call_run(call, out.data_ptr(), lse_ptr, base, scratch_bytes, words.data_ptr(), words.numel(),
                              status_ptr, stream)
     _check(rc, "sa_call_attend")
@@ -431,7 +434,7 @@ def run_call(q: torch.Tensor, k: torch.Tensor, mask: torch.Tensor, call: bytes, 
 
 def fused_call(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, mask: torch.Tensor, block_q: int, block_k: int,
                with_lse: bool, splits: int, check_status: bool):
-    """Both stages of a call in one native call: (out, lse or None), or None where :func:`plan_call` says None."""
+    """Both stages of a call over one scratch: (out, lse or None), or None where :func:`plan_call` says None."""
     planned = plan_call(q, k, v, mask, block_q, block_k, splits)
     return None if planned is None else run_call(q, k, mask, *planned, block_k, with_lse, check_status)[:2]
 

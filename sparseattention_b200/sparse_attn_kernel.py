@@ -123,9 +123,11 @@ def sparse_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, mask: to
 
     Gradients: the call is differentiable with respect to q, k and v (``out.backward(...)``; also through
     ``lse``).  The backward pass -- which the reference does not have -- recomputes P from the forward's
-    log-sum-exp and walks the same lists (CUDA-core kernels, fp32 math).  With caller-supplied lists for
-    BLOCK_Q = 32 / 64 the forward then runs the generic kernel on exactly those lists, so that forward and
-    backward see the same tiles.
+    log-sum-exp and walks the same lists: fp16 / bf16 with D in {64,128} on the tensor cores, with P and dS rounded to
+    the input type and fp32 sums (tcgen05 for lists at 128 query rows, warp-level MMA for caller lists at other heights),
+    everything else on the CUDA cores in fp32.  With caller-supplied lists for BLOCK_Q = 32 / 64 the forward then runs
+    the generic kernel on exactly those lists, so that forward and backward see the same tiles.  ``check_status``
+    holds for the backward of the call too.
 
     ``cache=True`` (with no ``mask_metadata``) keeps the lists and the packed plane of this mask and
     reuses them on every later call that passes the same mask memory, unmodified, with the same block
@@ -149,7 +151,7 @@ def sparse_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, mask: to
     # a backward pass needs the log-sum-exp of the forward
     needs_grad = torch.is_grad_enabled() and (q.requires_grad or k.requires_grad or v.requires_grad)
     if mask_metadata is None and impl == "auto" and not cache and (splits is None or splits == 1):
-        # both stages in one native call; None: not a call it takes as it is, which the general path below does
+        # both stages planned at once over one scratch; None: not a call of that kind, which the general path below does
         if not needs_grad:
             fused = _native.fused_call(q, k, v, mask, int(BLOCK_Q), int(BLOCK_K), bool(return_lse), splits or 0,
                                        bool(check_status))
